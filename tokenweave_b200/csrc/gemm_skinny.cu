@@ -1,0 +1,412 @@
+// Products with few rows (decode steps, language-model heads): C[M,N] = A[M,K] * W[N,K]^T for M up to a few hundred.
+//
+// Such a product is bound by reading W once from memory, so the tile follows W and not A: 128 rows of W (64 gate and 64 up
+// rows of a gated product) are the M side of tcgen05.mma, and ALL rows of A, padded to 16, are its N side. A stage of the
+// pipeline is then 16 KB of weights and M x 128 bytes of activations, where a tile of 128 rows of A would fill two thirds of
+// it with padding, and a narrow N (4096 outputs are 32 tiles) is spread over the chip by cutting K: a thread-block cluster of
+// up to 8 CTAs shares a tile, each CTA sums its part of K in TMEM, and the parts are added through distributed shared memory
+// in the order of the ranks - no workspace in global memory, no counters, the same result on every run.
+//
+//   warp 0      TMA producer (weights with an evict-first policy: they are read once)
+//   warp 1      MMA issuer
+//   warps 2..5  accumulators TMEM -> shared memory (fp32, where the stages were), then all threads of the cluster add the
+//               parts and run the epilogue on 8 outputs of one row each
+// What bounds it: memory. The down projection 4096x14336 of 48 rows takes 27 us (4.4 TB/s; 62 us with tiles of 128 rows of A,
+// which are 32 CTAs), a head of 128256x4096 164 us (6.4 TB/s), the gated 2x14336x4096 43 us (5.5 TB/s; before 67 us).
+// TMEM is given back before a CTA waits for the others of its cluster, so waiting for it never waits for a cluster.
+// Every mbarrier wait is bounded; after a timeout the CTA still takes part in the cluster's barriers.
+#include "tw_common.cuh"
+#include "tw_host.h"
+#include "tw_kernels.h"
+
+namespace tw {
+
+constexpr int SK_ROWS = 128;            // rows of W per tile
+constexpr int SK_THREADS = 192;
+constexpr int SK_MAX_STAGES = 16;
+constexpr int SK_MAX_TOKENS = 256;
+constexpr int SK_W_BYTES = SK_ROWS * 128;   // a k-block is 128 bytes of every row: 64 bf16 or 128 e4m3
+
+struct SkinnyParams {
+  __nv_bfloat16* C;
+  long long ldc;
+  const __nv_bfloat16* bias;
+  const float* row_scale;
+  const float* col_scale;   // fp8: per-output-channel scale (may be null)
+  int M, N;
+  int num_kb;
+  int tn;                   // rows of A, padded to 16
+  int stages;
+  int split;                // CTAs of a cluster: parts of K
+  int tmem_cols;
+  int up_row_offset;
+  GemmActs acts;
+  uint32_t* status;
+};
+
+__device__ __forceinline__ uint32_t cluster_rank() {
+  uint32_t r;
+  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+  return r;
+}
+__device__ __forceinline__ void cluster_sync_all() {
+  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+__device__ __forceinline__ float4 ld_cluster_f4(uint32_t local_addr, uint32_t rank) {
+  float4 v;
+  asm volatile(
+      "{\n\t.reg .u32 a;\n\tmapa.shared::cluster.u32 a, %4, %5;\n\t"
+      "ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [a];\n\t}"
+      : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w)
+      : "r"(local_addr), "r"(rank)
+      : "memory");
+  return v;
+}
+
+template <bool GLU, bool FP8, int KBS>
+__global__ void __launch_bounds__(SK_THREADS, 2)
+gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmW, const SkinnyParams p) {
+  constexpr int BK = FP8 ? 128 : 64;
+  constexpr int OUT = GLU ? SK_ROWS / 2 : SK_ROWS;      // output columns per tile
+  const int kb_bytes = SK_W_BYTES + p.tn * 128;
+
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
+  __shared__ uint64_t full_bar[SK_MAX_STAGES], empty_bar[SK_MAX_STAGES], acc_bar;
+  __shared__ uint32_t tmem_slot;
+  __shared__ volatile int abort_flag;
+
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int part = p.split > 1 ? static_cast<int>(cluster_rank()) : 0;
+  const int tile = blockIdx.x / p.split;
+  const int kb0 = static_cast<int>(static_cast<long long>(p.num_kb) * part / p.split);
+  const int kb1 = static_cast<int>(static_cast<long long>(p.num_kb) * (part + 1) / p.split);
+
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < p.stages; ++s) {
+      mbar_init(&full_bar[s], 1);
+      mbar_init(&empty_bar[s], 1);
+    }
+    mbar_init(&acc_bar, 1);
+    abort_flag = 0;
+    mbar_fence_init();
+    tma_prefetch_desc(&tmA);
+    tma_prefetch_desc(&tmW);
+  }
+  if (warp == 1) {
+    tmem_alloc(&tmem_slot, p.tmem_cols);
+    tmem_relinquish();
+  }
+  tc_fence_before_sync();
+  __syncthreads();
+  tc_fence_after_sync();
+  const uint32_t tmem = tmem_slot;
+
+  // One thread of each issuing warp, chosen by elect.sync and not by its lane number: the compiler then knows that a single
+  // thread runs the loop, and one CTA gets through a k-block in 0.17 us instead of 0.31.
+  if (warp == 0) {
+    if (elect_one()) {
+      const uint64_t once = policy_evict_first();
+      int stage = 0;
+      uint32_t phase = 0;
+      for (int kb = kb0; kb < kb1; kb += KBS) {
+        if (!mbar_wait(&empty_bar[stage], phase ^ 1)) {
+          report_error(p.status, TW_ERR_MBAR_TIMEOUT);
+          abort_flag = 1;
+          break;
+        }
+        uint8_t* sw = smem + stage * KBS * kb_bytes;
+        mbar_expect_tx(&full_bar[stage], KBS * kb_bytes);
+#pragma unroll
+        for (int h = 0; h < KBS; ++h, sw += kb_bytes) {
+          const int x = min(kb + h, kb1) * BK;    // past the part's end: loaded, not multiplied (past K: zeros)
+          if (GLU) {
+            tma_load_2d_hint(sw, &tmW, &full_bar[stage], x, tile * OUT, once);
+            tma_load_2d_hint(sw + SK_W_BYTES / 2, &tmW, &full_bar[stage], x, tile * OUT + p.up_row_offset, once);
+          } else {
+            tma_load_2d_hint(sw, &tmW, &full_bar[stage], x, tile * OUT, once);
+          }
+          tma_load_2d(sw + SK_W_BYTES, &tmA, &full_bar[stage], x, 0);
+        }
+        if (++stage == p.stages) { stage = 0; phase ^= 1; }
+      }
+    }
+  } else if (warp == 1) {
+    if (elect_one()) {
+      const uint32_t idesc = FP8 ? make_idesc_e4m3(SK_ROWS, p.tn) : make_idesc_bf16(SK_ROWS, p.tn, 0, 0);
+      int stage = 0;
+      uint32_t phase = 0;
+      for (int kb = kb0; kb < kb1; kb += KBS) {
+        if (!mbar_wait(&full_bar[stage], phase)) {
+          report_error(p.status, TW_ERR_MBAR_TIMEOUT);
+          abort_flag = 1;
+          break;
+        }
+        tc_fence_after_sync();
+        const uint32_t sw = smem_u32(smem + stage * KBS * kb_bytes);
+#pragma unroll
+        for (int h = 0; h < KBS; ++h) {
+          if (KBS > 1 && kb + h >= kb1) break;
+          const uint64_t w_desc = make_smem_desc_sw128(sw + h * kb_bytes, 16, 1024);
+          const uint64_t a_desc = make_smem_desc_sw128(sw + h * kb_bytes + SK_W_BYTES, 16, 1024);
+#pragma unroll
+          for (int k = 0; k < 4; ++k) {     // 32 bytes further along K: +2 in the descriptor's 16-byte units
+            const uint32_t acc = (kb != kb0 || h != 0 || k != 0) ? 1u : 0u;
+            if (FP8) umma_ss_f8(tmem, w_desc + 2 * k, a_desc + 2 * k, idesc, acc);
+            else umma_ss(tmem, w_desc + 2 * k, a_desc + 2 * k, idesc, acc);
+          }
+        }
+        umma_commit(&empty_bar[stage]);
+        if (++stage == p.stages) { stage = 0; phase ^= 1; }
+      }
+      umma_commit(&acc_bar);
+    }
+  } else {
+    // accumulators -> shared memory, [row of A][row of W]: lanes are rows of W, so a warp writes 128 bytes in a row
+    if (!mbar_wait(&acc_bar, 0)) {
+      report_error(p.status, TW_ERR_MBAR_TIMEOUT);
+      abort_flag = 1;
+    }
+    tc_fence_after_sync();
+    const int q = warp & 3;
+    float* dst = reinterpret_cast<float*>(smem) + q * 32 + lane;
+    const uint32_t src = tmem + (static_cast<uint32_t>(q * 32) << 16);
+    if (!abort_flag) {
+#pragma unroll 1
+      for (int c = 0; c < p.tn; c += 16) {
+        uint32_t v[16];
+        tmem_ld_32x16(src + c, v);
+        tmem_wait_ld();
+#pragma unroll
+        for (int j = 0; j < 16; ++j) dst[(c + j) * SK_ROWS] = __uint_as_float(v[j]);
+      }
+    }
+    tc_fence_before_sync();
+  }
+  if (abort_flag) {                         // copies in flight land before shared memory is reused or released
+    const uint64_t t0 = globaltimer_ns();
+    while (globaltimer_ns() - t0 < 200000ull) __nanosleep(1000);
+  }
+  __syncthreads();
+  if (warp == 1) {
+    tc_fence_after_sync();
+    tmem_dealloc(tmem, p.tmem_cols);
+  }
+  if (p.split > 1) {
+    __syncwarp();
+    cluster_sync_all();
+  }
+
+  // ---- sums of the parts and epilogue: 8 neighbouring outputs of one row at a time ----
+  const uint32_t part0 = smem_u32(smem);
+  constexpr int GROUPS = OUT / 8;
+  const int items = p.M * GROUPS;
+  const int n_tile = tile * OUT;
+  for (int i = part * SK_THREADS + threadIdx.x; i < items; i += p.split * SK_THREADS) {
+    const int t = i / GROUPS, g = i % GROUPS;
+    const int n = n_tile + g * 8;
+    if (n >= p.N) continue;
+    float v[8], u[8];
+#pragma unroll
+    for (int e = 0; e < 8; ++e) v[e] = u[e] = 0.f;
+    const uint32_t at = part0 + (t * SK_ROWS + g * 8) * 4;
+    for (int s = 0; s < p.split; ++s) {
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        float4 a;
+        if (p.split > 1) a = ld_cluster_f4(at + h * 16, s);
+        else a = *reinterpret_cast<const float4*>(smem + (t * SK_ROWS + g * 8) * 4 + h * 16);
+        v[4 * h] += a.x; v[4 * h + 1] += a.y; v[4 * h + 2] += a.z; v[4 * h + 3] += a.w;
+        if (GLU) {
+          if (p.split > 1) a = ld_cluster_f4(at + OUT * 4 + h * 16, s);
+          else a = *reinterpret_cast<const float4*>(smem + (t * SK_ROWS + OUT + g * 8) * 4 + h * 16);
+          u[4 * h] += a.x; u[4 * h + 1] += a.y; u[4 * h + 2] += a.z; u[4 * h + 3] += a.w;
+        }
+      }
+    }
+    const float rs = p.row_scale != nullptr ? p.row_scale[t] : 1.f;
+    float r[8];
+#pragma unroll
+    for (int e = 0; e < 8; ++e) {
+      const int c = min(n + e, p.N - 1);
+      if (GLU) {
+        float x = v[e], y = u[e];
+        if (FP8) {
+          x *= rs;
+          if (p.col_scale != nullptr) {
+            x *= p.col_scale[c];
+            y *= p.col_scale[p.up_row_offset + c];
+          }
+          r[e] = x / (1.f + __expf(-x)) * y * rs;
+        } else if (p.acts.glu == GLU_GELU_TANH) {
+          r[e] = epi_gelu_tanh(x) * y * rs;
+        } else if (p.acts.glu == GLU_CLAMPED) {
+          r[e] = epi_clamped(x * rs, y * rs, p.acts.limit, p.acts.alpha);
+        } else {
+          r[e] = x / (1.f + __expf(-x)) * y * rs;
+        }
+      } else {
+        float x = v[e];
+        if (FP8) {
+          x *= p.col_scale != nullptr ? rs * p.col_scale[c] : rs;
+          if (p.bias != nullptr) x += __bfloat162float(p.bias[c]);
+        } else {
+          if (p.bias != nullptr) x += __bfloat162float(p.bias[c]);
+          if (p.acts.col_act != 0 && c >= p.acts.col_begin && c < p.acts.col_end) {
+            const float z = fmaxf(x, 0.f);
+            x = p.acts.col_act == COL_RELU2 ? z * z : epi_silu(x);
+          }
+          x *= rs;
+        }
+        r[e] = x;
+      }
+    }
+    __nv_bfloat16* crow = p.C + static_cast<long long>(t) * p.ldc + n;
+    if (n + 8 <= p.N) {
+      *reinterpret_cast<uint4*>(crow) = make_uint4(pack_bf16x2(r[0], r[1]), pack_bf16x2(r[2], r[3]),
+                                                   pack_bf16x2(r[4], r[5]), pack_bf16x2(r[6], r[7]));
+    } else {
+#pragma unroll
+      for (int e = 0; e < 8; ++e)
+        if (n + e < p.N) crow[e] = __float2bfloat16_rn(r[e]);
+    }
+  }
+  if (p.split > 1) {
+    __syncwarp();
+    cluster_sync_all();                     // the others may still read this CTA's part
+  }
+}
+
+template <bool GLU, bool FP8, int KBS>
+static int launch_skinny(const CUtensorMap& tmA, const CUtensorMap& tmW, const SkinnyParams& p, int tiles, int smem,
+                         cudaStream_t stream) {
+  auto kern = gemm_skinny_kernel<GLU, FP8, KBS>;
+  static thread_local int configured_dev = -1;
+  int dev = 0;
+  cudaGetDevice(&dev);
+  if (configured_dev != dev) {
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 226 * 1024);
+    if (e != cudaSuccess) {
+      set_last_error("cudaFuncSetAttribute(smem) failed: %s", cudaGetErrorString(e));
+      return 1;
+    }
+    configured_dev = dev;
+  }
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(tiles * p.split);
+  cfg.blockDim = dim3(SK_THREADS);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = p.split;
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = p.split > 1 ? 1 : 0;
+  cudaError_t e = cudaLaunchKernelEx(&cfg, kern, tmA, tmW, p);
+  if (e == cudaSuccess) e = cudaGetLastError();
+  if (e != cudaSuccess) {
+    set_last_error("gemm launch failed: %s", cudaGetErrorString(e));
+    return 1;
+  }
+  return 0;
+}
+
+// Which products come here; the rest keeps the tiles of 128 or 256 rows of A. Measured on B200, weights from memory (us,
+// tiles of A -> this kernel; the former also with elect.sync):
+//   up to 80 rows: always. 4096x14336 62 -> 27 (48 rows), 8192x28672 124 -> 79, gated 2x14336x4096 67 -> 43, fp8 5120x25600
+//     58 -> 34 (32 rows)
+//   up to 160 rows: gated 2x28672x8192 183 -> 159 (96), 257 -> 182 (160). Not up to 128 rows where A is one tile of theirs and
+//     the tiles of W are many waves here, each of which reads A again from L2: head 128256x4096 180 -> 185 (96) and 184 -> 197
+//     (128), gated 2x25600x5120 95 -> 112 (128); but gated 2x14336x4096 55 -> 52 (128)
+//   up to 256 rows: only one CTA fits an SM, so only where cutting K fills the chip and the parts are long enough to pay for
+//     adding 100 KB of sums: 8192x28672 126 -> 95 (200), 128 -> 109 (256), 4096x14336 63 -> 34; but 10240x8192 47 -> 55 and
+//     6144x4096 23 -> 26 (256)
+bool gemm_skinny_takes(bool fp8, int M, int N, int K, bool glu) {
+  if (M <= 80) return true;
+  if (M > SK_MAX_TOKENS) return false;
+  const int out = glu ? SK_ROWS / 2 : SK_ROWS;
+  const int tiles = (N + out - 1) / out, sms = device_sm_count();
+  const int num_kb = (K + (fp8 ? 127 : 63)) / (fp8 ? 128 : 64);
+  if (M <= 160) return M > 128 || tiles <= (M <= 112 ? 4 : 2) * sms;
+  return 2 * tiles <= sms && num_kb >= (M <= 208 ? 64 : 128);
+}
+
+int gemm_skinny(bool fp8, const void* A, long long lda, const void* W, long long ldw, long long rows_w, void* C, long long ldc,
+                const void* bias, const float* row_scale, const float* col_scale, int M, int N, int K, int glu,
+                int up_row_offset, const GemmActs& acts, uint32_t* status, cudaStream_t stream) {
+  const int esz = fp8 ? 1 : 2, bk = fp8 ? 128 : 64;
+  SkinnyParams p;
+  p.tn = (M + 15) / 16 * 16;
+  p.num_kb = (K + bk - 1) / bk;
+  const int out = glu ? SK_ROWS / 2 : SK_ROWS;
+  const int tiles = (N + out - 1) / out;
+  const int sms = device_sm_count();
+  const int kb_bytes = SK_W_BYTES + p.tn * 128;
+  // Two CTAs per SM (one loads while the other starts or ends) where three stages of both fit: up to 160 rows.
+  // Parts of K: doubled until the CTAs cover 0.6 of the SMs, half of them from 64 rows on, where the sums to be added weigh
+  // more; more parts than that only add sums (48 rows, 6144x4096 in 2 / 4 parts: 14.8 / 16.2 us; 4096x4096 in 4 / 8: 12.1 /
+  // 15.0; 128 rows, 5120x8192 in 2 / 4: 26.6 / 28.3). At least four k-blocks each, and never a second wave.
+  // fp8 is not cut: the sums of one accumulator over all of K are bit for bit those of the tiles of A, and a last bit that
+  // differs moves the scale with which the next layer rounds a whole row to eight bits.
+  const int two = 110 * 1024, one = 220 * 1024;
+  const bool pairs = 3 * kb_bytes <= two;
+  const int slots = pairs ? 2 * sms : sms;
+  const int enough = sms * (M < 64 ? 6 : 5) / 10;
+  int split = 1;
+  while (!fp8 && split < 8 && tiles * split < enough && tiles * split * 2 <= slots && p.num_kb / (split * 2) >= 4) split *= 2;
+  p.split = split;
+  // One CTA per SM sets the pace itself: two k-blocks per stage halve its waits, as long as four stages are left
+  // (fp8 5120x25600, 1 row: 37 -> 30 us; 100 rows, three stages: 46 -> 55 us).
+  const bool alone = !pairs || tiles * split <= sms;
+  const int kbs = alone && 8 * kb_bytes <= one ? 2 : 1;
+  p.stages = min(SK_MAX_STAGES, (alone ? one : two) / (kbs * kb_bytes));
+  const int dump = SK_ROWS * p.tn * 4;
+  int smem = p.stages * kbs * kb_bytes;
+  if (smem < dump) smem = dump;
+  if (smem < 80 * 1024) smem = 80 * 1024;   // at most two CTAs per SM: none waits for another's TMEM
+  smem += 1024;
+  p.tmem_cols = 32;
+  while (p.tmem_cols < p.tn) p.tmem_cols *= 2;
+
+  CUtensorMap tmA, tmW;
+  {
+    uint64_t dims[2] = {(uint64_t)K, (uint64_t)M};
+    uint64_t strides[1] = {(uint64_t)lda * esz};
+    uint32_t box[2] = {(uint32_t)bk, (uint32_t)p.tn};
+    if (!(fp8 ? make_tensor_map_u8(&tmA, A, 2, dims, strides, box) : make_tensor_map_bf16(&tmA, A, 2, dims, strides, box)))
+      return 1;
+  }
+  {
+    uint64_t dims[2] = {(uint64_t)K, (uint64_t)rows_w};
+    uint64_t strides[1] = {(uint64_t)ldw * esz};
+    uint32_t box[2] = {(uint32_t)bk, (uint32_t)out};
+    if (!(fp8 ? make_tensor_map_u8(&tmW, W, 2, dims, strides, box) : make_tensor_map_bf16(&tmW, W, 2, dims, strides, box)))
+      return 1;
+  }
+  p.C = reinterpret_cast<__nv_bfloat16*>(C);
+  p.ldc = ldc;
+  p.bias = reinterpret_cast<const __nv_bfloat16*>(bias);
+  p.row_scale = row_scale;
+  p.col_scale = col_scale;
+  p.M = M;
+  p.N = N;
+  p.up_row_offset = up_row_offset;
+  p.acts = acts;
+  p.status = status;
+  if (kbs == 2) {
+    if (fp8)
+      return glu ? launch_skinny<true, true, 2>(tmA, tmW, p, tiles, smem, stream)
+                 : launch_skinny<false, true, 2>(tmA, tmW, p, tiles, smem, stream);
+    return glu ? launch_skinny<true, false, 2>(tmA, tmW, p, tiles, smem, stream)
+               : launch_skinny<false, false, 2>(tmA, tmW, p, tiles, smem, stream);
+  }
+  if (fp8)
+    return glu ? launch_skinny<true, true, 1>(tmA, tmW, p, tiles, smem, stream)
+               : launch_skinny<false, true, 1>(tmA, tmW, p, tiles, smem, stream);
+  return glu ? launch_skinny<true, false, 1>(tmA, tmW, p, tiles, smem, stream)
+             : launch_skinny<false, false, 1>(tmA, tmW, p, tiles, smem, stream);
+}
+
+}  // namespace tw

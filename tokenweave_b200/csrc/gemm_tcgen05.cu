@@ -470,6 +470,12 @@ static GemmPlan choose_plan(int M, int N, int K, int sms, bool swiglu, bool grou
   return best;
 }
 
+// gemm_skinny.cu: tiles of 128 rows of the weights and all rows of A
+bool gemm_skinny_takes(bool fp8, int M, int N, int K, bool glu);
+int gemm_skinny(bool fp8, const void* A, long long lda, const void* W, long long ldw, long long rows_w, void* C, long long ldc,
+                const void* bias, const float* row_scale, const float* col_scale, int M, int N, int K, int glu,
+                int up_row_offset, const GemmActs& acts, uint32_t* status, cudaStream_t stream);
+
 }  // namespace tw
 
 using namespace tw;
@@ -518,6 +524,11 @@ static int gemm_dispatch(bool fp8, const void* A, long long lda, const void* B, 
   if (tile_expert != nullptr && group_tile_rows == 256 && sms >= 2)
     return tw_gemm_pair(fp8, A, lda, B, ldb, rows_b, C, ldc, bias, row_scale, col_scale, M, N, K, swiglu,
                         up_row_offset, 256, sms, tile_expert, num_m_tiles_dev, n_per_expert, &acts, status, stream);
+  // a budget of SMs or a forced tile means the persistent kernels; tuned hints were taken among those only
+  if (tile_expert == nullptr && max_ctas <= 0 && g_bn_override == 0 && g_kernel_override == 0 &&
+      gemm_skinny_takes(fp8, M, N, K, swiglu != 0))
+    return gemm_skinny(fp8, A, lda, B, ldb, rows_b, C, ldc, bias, row_scale, col_scale, M, N, K, swiglu, up_row_offset, acts,
+                       status, stream);
   // the cost model sees k-blocks: an fp8 problem has K / 128 of them
   GemmPlan plan = choose_plan(M, N, fp8 ? K / 2 : K, sms, swiglu != 0, tile_expert != nullptr);
   if (plan_hint > 0) {
