@@ -175,7 +175,7 @@ attn_decode_tc_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_cons
 
   if (warp == 0) {
     // ---------------- TMA producer ----------------
-    if (lane == 0 && n_tiles > 0) {
+    if (n_tiles > 0 && elect_one()) {
       tma_prefetch_desc(&tmK);
       tma_prefetch_desc(&tmV);
       const int pages_per_tile = DTC_BN / p.page;
@@ -207,7 +207,7 @@ attn_decode_tc_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_cons
     }
   } else if (warp == 1) {
     // ---------------- MMA issuer ----------------
-    if (lane == 0 && n_tiles > 0) {
+    if (n_tiles > 0 && elect_one()) {
       const uint32_t q_addr = smem_u32(smem + DTC_OFF_Q);
       bool ok = mbar_wait(q_ready, 0);
       auto issue_s = [&](int j) {
@@ -608,7 +608,7 @@ attn_decode_tc_persistent_kernel(const __grid_constant__ CUtensorMap tmK, const 
 
   if (warp == 0) {
     // ---------------- TMA producer: tiles of all items of this CTA, back to back ----------------
-    if (lane == 0) {
+    if (elect_one()) {
       tma_prefetch_desc(&tmK);
       tma_prefetch_desc(&tmV);
       const int pages_per_tile = DTC_BN / p.page;
@@ -652,7 +652,7 @@ attn_decode_tc_persistent_kernel(const __grid_constant__ CUtensorMap tmK, const 
     }
   } else if (warp == 1) {
     // ---------------- MMA issuer ----------------
-    if (lane == 0) {
+    if (elect_one()) {
       const uint32_t q_addr = smem_u32(smem + DTP_OFF_Q);
       uint32_t jt = 0, items_done = 0;
       bool ok = true;

@@ -116,7 +116,7 @@ attn_prefill_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
 
   if (warp == 0) {
     // ---------------- TMA producer ----------------
-    if (lane == 0 && n_tiles > 0) {
+    if (n_tiles > 0 && elect_one()) {
       tma_prefetch_desc(&tmQ);
       tma_prefetch_desc(&tmK);
       tma_prefetch_desc(&tmV);
@@ -154,7 +154,7 @@ attn_prefill_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
     }
   } else if (warp == 1) {
     // ---------------- MMA issuer ----------------
-    if (lane == 0 && n_tiles > 0) {
+    if (n_tiles > 0 && elect_one()) {
       const uint32_t q_addr = smem_u32(smem + S::OFF_Q);
       const uint32_t p_addr = smem_u32(smem + S::OFF_P);
       bool ok = mbar_wait(q_full, 0);
@@ -429,7 +429,7 @@ attn_prefill_pair_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_c
 
   if (warp == 0) {
     // ---------------- TMA producer ----------------
-    if (lane == 0 && n_tiles > 0) {
+    if (n_tiles > 0 && elect_one()) {
       tma_prefetch_desc(&tmQ);
       tma_prefetch_desc(&tmK);
       tma_prefetch_desc(&tmV);
@@ -462,7 +462,7 @@ attn_prefill_pair_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_c
     }
   } else if (warp == 1) {
     // ---------------- MMA issuer ----------------
-    if (lane == 0 && n_tiles > 0) {
+    if (n_tiles > 0 && elect_one()) {
       bool ok = mbar_wait(q_full, 0);
       // S_g = Q_g K_j^T; K_j is stream element 2j. `last` releases the slot (both heads have read it).
       auto issue_qk = [&](int g, int j, bool last) {

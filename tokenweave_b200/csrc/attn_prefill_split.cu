@@ -169,7 +169,7 @@ attn_prefill_split_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_
 
   if (warp == 0) {
     // ---------------- TMA producer ----------------
-    if (lane == 0) {
+    if (elect_one()) {
       tma_prefetch_desc(&tmQ);
       tma_prefetch_desc(&tmK);
       tma_prefetch_desc(&tmV);
@@ -222,7 +222,7 @@ attn_prefill_split_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_
     }
   } else if (warp == 1) {
     // ---------------- MMA issuer ----------------
-    if (lane == 0) {
+    if (elect_one()) {
       uint32_t e[2] = {0u, 0u};           // ring elements consumed so far, per group
       uint32_t cnt[2] = {0u, 0u};         // key tiles whose P V has been issued, per group
       const uint32_t q_addr = smem_u32(smem + S::OFF_Q);

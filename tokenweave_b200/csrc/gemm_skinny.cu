@@ -329,6 +329,7 @@ bool gemm_skinny_takes(bool fp8, int M, int N, int K, bool glu) {
   const int out = glu ? SK_ROWS / 2 : SK_ROWS;
   const int tiles = (N + out - 1) / out, sms = device_sm_count();
   const int num_kb = (K + (fp8 ? 127 : 63)) / (fp8 ? 128 : 64);
+  if (fp8 && M > 112 && tiles < sms) return false;   // not cut (below): too few CTAs once the MMAs are this wide
   if (M <= 160) return M > 128 || tiles <= (M <= 112 ? 4 : 2) * sms;
   return 2 * tiles <= sms && num_kb >= (M <= 208 ? 64 : 128);
 }

@@ -144,7 +144,7 @@ latent_prefill_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
 
   if (warp == 0) {
     // ---------------- TMA producer ----------------
-    if (lane == 0) {
+    if (elect_one()) {
       tma_prefetch_desc(&tmQ);
       tma_prefetch_desc(&tmK);
       tma_prefetch_desc(&tmR);
@@ -204,7 +204,7 @@ latent_prefill_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
     }
   } else if (warp == 1) {
     // ---------------- MMA issuer ----------------
-    if (lane == 0) {
+    if (elect_one()) {
       uint32_t ek[2] = {0u, 0u};          // key tiles whose scores have been issued, per group
       uint32_t cnt[2] = {0u, 0u};         // key tiles whose P V has been issued, per group
       const uint32_t q_addr = smem_u32(smem + S::OFF_Q);
