@@ -12,7 +12,7 @@ pytestmark = pytest.mark.gpu
 BF = torch.bfloat16
 
 # 128 outputs: 1 tile; 4096: 32 tiles, 4 parts; 5000: ragged; K 264 and 72: a k-block that ends early, no cut
-SHAPES = [(128, 72), (136, 264), (1000, 2056), (4096, 4096), (5000, 1024), (20000, 512)]
+SHAPES = [(128, 72), (136, 264), (1000, 2056), (4096, 4096), (5000, 1024), (20000, 512), (19336, 8200)]
 
 
 def rnd(*shape, scale=1.0):
@@ -34,7 +34,7 @@ def _status_clean():
 
 
 @pytest.mark.parametrize("N,K", SHAPES)
-@pytest.mark.parametrize("M", [1, 16, 17, 63, 64, 80, 81, 128, 129, 160, 161, 208, 209, 256])
+@pytest.mark.parametrize("M", [1, 16, 17, 63, 64, 80, 81, 112, 113, 128, 129, 160, 161, 208, 209, 224, 225, 256])
 def test_plain(M, N, K):
     a, w, bias, rs = rnd(M, K), rnd(N, K, scale=K ** -0.5), rnd(N), torch.rand(M, device="cuda") + 0.5
     big = torch.zeros(M + 1, N + 8 + -N % 8, device="cuda", dtype=BF)
@@ -45,7 +45,7 @@ def test_plain(M, N, K):
 
 
 @pytest.mark.parametrize("N,K", [(64, 72), (200, 264), (4096, 1024), (14336, 512)])
-@pytest.mark.parametrize("M", [1, 33, 100, 200])
+@pytest.mark.parametrize("M", [1, 33, 100, 140, 200, 224])
 def test_gated_and_activations(M, N, K):
     a, w = rnd(M, K), rnd(2 * N, K, scale=K ** -0.5)
     g, u = (a.float() @ w.float().T).chunk(2, -1)
@@ -61,8 +61,8 @@ def test_gated_and_activations(M, N, K):
     near(ops.gemm(a, w, col_act=("relu2", lo, hi)), want)
 
 
-@pytest.mark.parametrize("N,K", [(128, 144), (1000, 1040), (4096, 4096), (24, 528)])
-@pytest.mark.parametrize("M", [1, 31, 96, 160, 208])
+@pytest.mark.parametrize("N,K", [(128, 144), (1000, 1040), (4096, 4096), (24, 528), (20000, 528)])
+@pytest.mark.parametrize("M", [1, 31, 96, 150, 160, 208])
 def test_fp8(M, N, K):
     aq, a_s = ops.quant_fp8(rnd(M, K))
     wq, w_s = ops.quant_fp8(rnd(2 * N, K, scale=K ** -0.5))
@@ -73,3 +73,15 @@ def test_fp8(M, N, K):
     near(ops.gemm_fp8(aq, wq, a_s, w_s, swiglu=True), torch.nn.functional.silu(g) * u)
     raw = aq.float() @ wq.float().T
     near(ops.gemm_fp8(aq, wq, None, None), raw)
+
+
+@pytest.mark.parametrize("V,padded,K", [(512, 512, 256), (2000, 2048, 264), (1003, 1024, 128), (32064, 32064, 512)])
+@pytest.mark.parametrize("M", [1, 24, 100, 130, 200, 256, 257])
+def test_logits_are_the_converted_product(M, V, padded, K):
+    a, w = rnd(M, K), rnd(padded, K, scale=K ** -0.5)
+    for scale in (1.0, 0.37):
+        got = ops.head_logits(a, w, V, scale)
+        assert got.dtype == torch.float32 and got.shape == (M, V)
+        near(got / scale, a.float() @ w.float().T[:, :V])
+        if scale == 1.0:
+            assert torch.equal(got, got.to(BF).float())

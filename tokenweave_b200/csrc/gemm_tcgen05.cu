@@ -471,10 +471,11 @@ static GemmPlan choose_plan(int M, int N, int K, int sms, bool swiglu, bool grou
 }
 
 // gemm_skinny.cu: tiles of 128 rows of the weights and all rows of A
-bool gemm_skinny_takes(bool fp8, int M, int N, int K, bool glu);
-int gemm_skinny(bool fp8, const void* A, long long lda, const void* W, long long ldw, long long rows_w, void* C, long long ldc,
+bool gemm_skinny_takes(bool fp8, bool cut, int M, int N, int K, bool glu);
+int gemm_skinny(bool fp8, bool cut, const void* A, long long lda, const void* W, long long ldw, long long rows_w, void* C, long long ldc,
                 const void* bias, const float* row_scale, const float* col_scale, int M, int N, int K, int glu,
-                int up_row_offset, const GemmActs& acts, uint32_t* status, cudaStream_t stream);
+                int up_row_offset, const GemmActs& acts, uint32_t* status, cudaStream_t stream, float* logits = nullptr,
+                float logit_scale = 1.f);
 
 }  // namespace tw
 
@@ -507,8 +508,10 @@ static int gemm_dispatch(bool fp8, const void* A, long long lda, const void* B, 
   if (swiglu && acts.glu == 0) acts.glu = swiglu;
   // group_tile_rows: rows per entry of tile_expert (grouped mode). 256: the caller padded every expert to 256
   // rows, so the CTA-pair kernel can take the groups; 128: single-CTA tiles.
-  // plan_hint: 0 = cost model; otherwise kernel * 1000 + tile width (kernel 1 = single-CTA tiles,
+  // plan_hint: 10000 and more = K is not cut (one sum per result); the rest of it 0 = cost model; otherwise kernel * 1000 + tile width (kernel 1 = single-CTA tiles,
   // 2 = CTA pairs), as produced by the tuning table.
+  const bool cut = plan_hint < 10000 && !fp8;
+  plan_hint %= 10000;
   if (M <= 0 || N <= 0 || K <= 0) return 0;
   const int in_align = fp8 ? 16 : 8;   // 16 bytes of operand elements
   if ((K % in_align) != 0 || (lda % in_align) != 0 || (ldb % in_align) != 0 || (ldc % 8) != 0) {
@@ -526,8 +529,8 @@ static int gemm_dispatch(bool fp8, const void* A, long long lda, const void* B, 
                         up_row_offset, 256, sms, tile_expert, num_m_tiles_dev, n_per_expert, &acts, status, stream);
   // a budget of SMs or a forced tile means the persistent kernels; tuned hints were taken among those only
   if (tile_expert == nullptr && max_ctas <= 0 && g_bn_override == 0 && g_kernel_override == 0 &&
-      gemm_skinny_takes(fp8, M, N, K, swiglu != 0))
-    return gemm_skinny(fp8, A, lda, B, ldb, rows_b, C, ldc, bias, row_scale, col_scale, M, N, K, swiglu, up_row_offset, acts,
+      gemm_skinny_takes(fp8, cut, M, N, K, swiglu != 0))
+    return gemm_skinny(fp8, cut, A, lda, B, ldb, rows_b, C, ldc, bias, row_scale, col_scale, M, N, K, swiglu, up_row_offset, acts,
                        status, stream);
   // the cost model sees k-blocks: an fp8 problem has K / 128 of them
   GemmPlan plan = choose_plan(M, N, fp8 ? K / 2 : K, sms, swiglu != 0, tile_expert != nullptr);

@@ -220,6 +220,9 @@ int tw_attn_decode_grouped(const void* q, long long ldq, const void* k_cache, co
                            int dp, int vp, float scale, const float* slopes, int sink, float out_scale, int window,
                            int keep, const float* key_bias, int chunk, const void* gate, long long ldg, int splits,
                            float* part_o, float* part_ml, uint32_t* status, cudaStream_t stream);
+int tw_gemm_logits_takes(int M, int N, int K);
+int tw_gemm_logits(const void* A, long long lda, const void* W, long long ldw, float* logits, long long ldc, float scale, int M,
+                   int N, int K, uint32_t* status, cudaStream_t stream);
 int tw_gemm_bf16_act(const void* A, long long lda, const void* B, long long ldb, void* C, long long ldc,
                      const void* bias, int M, int N, int K, int act, int act_begin, int act_end, int max_ctas, int plan_hint,
                      uint32_t* status, cudaStream_t stream);

@@ -71,15 +71,16 @@ class ParallelLMHead(nn.Module):
     def forward(self, hidden: torch.Tensor) -> torch.Tensor:
         """fp32 logits ``[rows, vocab_size]`` on every rank."""
         tp = get_tp()
+        if tp.world_size == 1:
+            return ops.head_logits(hidden, self.weight, self.vocab_size)
         local = ops.gemm(hidden, self.weight)
-        if tp.world_size > 1:
-            rows, cols = local.shape
-            gathered = torch.empty(tp.world_size * rows, cols, dtype=local.dtype, device=local.device)
-            if self.comm is not None:
-                self.comm.nccl_all_gather(gathered.view(-1), local.contiguous().view(-1))
-            else:
-                dist.all_gather_into_tensor(gathered, local.contiguous(), group=tp.group)
-            local = gathered.view(tp.world_size, rows, cols).permute(1, 0, 2).reshape(rows, -1)
+        rows, cols = local.shape
+        gathered = torch.empty(tp.world_size * rows, cols, dtype=local.dtype, device=local.device)
+        if self.comm is not None:
+            self.comm.nccl_all_gather(gathered.view(-1), local.contiguous().view(-1))
+        else:
+            dist.all_gather_into_tensor(gathered, local.contiguous(), group=tp.group)
+        local = gathered.view(tp.world_size, rows, cols).permute(1, 0, 2).reshape(rows, -1)
         return local[:, : self.vocab_size].float()
 
     def weight_loader(self, param: nn.Parameter, loaded: torch.Tensor, shard_id=None) -> None:

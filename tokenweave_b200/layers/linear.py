@@ -47,9 +47,10 @@ class _QuantizableLinear(nn.Module):
         self.weight_scale = scale
 
     def _gemm(self, x: torch.Tensor, out: Optional[torch.Tensor], *, bias=None, row_scale=None, swiglu=False,
-              max_ctas: int = 0) -> torch.Tensor:
+              max_ctas: int = 0, cut_k: bool = True) -> torch.Tensor:
         if self.weight_scale is None:
-            return ops.gemm(x, self.weight, out=out, bias=bias, row_scale=row_scale, swiglu=swiglu, max_ctas=max_ctas)
+            return ops.gemm(x, self.weight, out=out, bias=bias, row_scale=row_scale, swiglu=swiglu, max_ctas=max_ctas,
+                            cut_k=cut_k)
         if out is None:
             n = self.weight.shape[0] // 2 if swiglu else self.weight.shape[0]
             out = torch.empty(x.shape[0], n, dtype=x.dtype, device=x.device)
@@ -214,4 +215,5 @@ class PaddedLinear(_QuantizableLinear):
         self.weight.data[:t.shape[0], col:col + t.shape[1]].copy_(t)
 
     def forward(self, x: torch.Tensor, out: Optional[torch.Tensor] = None, max_ctas: int = 0) -> torch.Tensor:
-        return self._gemm(x, out, bias=self.bias, max_ctas=max_ctas)
+        # the polynomial activations of hybrid decoders magnify last bits: sums in one order whatever the batch
+        return self._gemm(x, out, bias=self.bias, max_ctas=max_ctas, cut_k=False)

@@ -32,6 +32,7 @@ import numpy as np
 import torch
 from torch import nn
 
+from .. import ops
 from ..config import ModelConfig
 from ..layers.attention import PREFILL_MIN_Q, AttentionMetadata
 from ..layers.linear import PaddedLinear, pad8
@@ -456,6 +457,8 @@ class HybridDecoder(nn.Module):
     @torch.inference_mode()
     def compute_logits(self, hidden_rows: torch.Tensor) -> torch.Tensor:
         """fp32 logits ``[rows, vocab]``."""
+        if self.head.weight_scale is None and self.head.bias is None:
+            return ops.head_logits(hidden_rows, self.head.weight, self.cfg.vocab_size, self.cfg.logit_scale)
         return self.head(hidden_rows)[:, : self.cfg.vocab_size].float() * self.cfg.logit_scale
 
     # ---- weights ---------------------------------------------------------------------------------------

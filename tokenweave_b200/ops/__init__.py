@@ -88,7 +88,7 @@ COL_ACTS = {"silu": 1, "relu2": 2}
 def gemm(a: torch.Tensor, w: torch.Tensor, out: Optional[torch.Tensor] = None, *,
          bias: Optional[torch.Tensor] = None, row_scale: Optional[torch.Tensor] = None, swiglu: bool = False,
          act: "str | tuple" = "silu", col_act: Optional[tuple[str, int, int]] = None, max_ctas: int = 0,
-         in_scale: Optional[torch.Tensor] = None,
+         in_scale: Optional[torch.Tensor] = None, cut_k: bool = True,
          tile_expert: Optional[torch.Tensor] = None,
          num_m_tiles: Optional[torch.Tensor] = None, n_per_expert: int = 0, tile_rows: int = 128) -> torch.Tensor:
     """``out = a @ w.T`` (+bias, *row_scale); with ``swiglu`` the weight is ``[gate; up]`` and the
@@ -98,7 +98,9 @@ def gemm(a: torch.Tensor, w: torch.Tensor, out: Optional[torch.Tensor] = None, *
     ``col_act`` = ("silu" or "relu2", begin, end): that activation on these columns of a plain product (behind the bias;
     relu2: the square of relu). Grouped mode (``tile_expert`` given): every ``tile_rows``-row
     tile of ``a`` multiplies the weight block of its expert, ``w`` being ``[E * n_per_expert, K]``;
-    ``tile_rows`` is 128 (single-CTA tiles) or 256 (experts padded to 256 rows: the groups run on CTA pairs)."""
+    ``tile_rows`` is 128 (single-CTA tiles) or 256 (experts padded to 256 rows: the groups run on CTA pairs).
+    ``cut_k`` False: one sum over all of K per result also for few rows, so that a row's result does not depend on how many
+    rows there are, to the last bit."""
     M, K = a.shape
     rows_b = w.shape[0]
     per_expert = n_per_expert if tile_expert is not None else rows_b
@@ -129,12 +131,13 @@ def gemm(a: torch.Tensor, w: torch.Tensor, out: Optional[torch.Tensor] = None, *
                      _row_stride(out), _p(bias), M, N, K, _stream())
         return out
     _check_bf16(a, w, out, bias)
+    whole = 0 if cut_k else 10000           # part of the launchers' plan hint
     if col_act is not None:
         if swiglu or row_scale is not None or tile_expert is not None:
             raise ValueError("an activation on a range of columns goes with a plain product")
         _native.call("tw_gemm_bf16_act", a.data_ptr(), _row_stride(a), w.data_ptr(), _row_stride(w), out.data_ptr(),
                      _row_stride(out), _p(bias), M, N, K, COL_ACTS[col_act[0]], int(col_act[1]), int(col_act[2]), max_ctas,
-                     gemm_table.lookup(M, N, K, False, max_ctas), status_word(a.device).data_ptr(), _stream(),
+                     gemm_table.lookup(M, N, K, False, max_ctas) + whole, status_word(a.device).data_ptr(), _stream(),
                      tag=f"[{M}x{N}x{K}+{col_act[0]}]" if _native._timing is not None else "")
         return out
     if swiglu and not isinstance(act, str):
@@ -146,7 +149,7 @@ def gemm(a: torch.Tensor, w: torch.Tensor, out: Optional[torch.Tensor] = None, *
                      out.data_ptr(), _row_stride(out), _p(in_scale), M, N, K, float(limit), float(alpha), per_expert // 2,
                      _p(tile_expert),
                      _p(num_m_tiles), per_expert, tile_rows, max_ctas,
-                     0 if grouped else gemm_table.lookup(M, N, K, True, max_ctas), status_word(a.device).data_ptr(),
+                     0 if grouped else gemm_table.lookup(M, N, K, True, max_ctas) + whole, status_word(a.device).data_ptr(),
                      _stream(), tag=f"[{'grouped ' if grouped else ''}{M}x{N}x{K}+clamped]" if _native._timing is not None else "")
         return out
     if tile_expert is not None and tile_rows == 256:
@@ -162,10 +165,25 @@ def gemm(a: torch.Tensor, w: torch.Tensor, out: Optional[torch.Tensor] = None, *
                  out.data_ptr(), _row_stride(out), _p(bias), _p(row_scale), M, N, K,
                  {"silu": 1, "gelu_tanh": 2}[act] if swiglu else 0,
                  per_expert // 2 if swiglu else 0, _p(tile_expert), _p(num_m_tiles), per_expert, max_ctas,
-                 0 if tile_expert is not None else gemm_table.lookup(M, N, K, swiglu, max_ctas),
+                 0 if tile_expert is not None else gemm_table.lookup(M, N, K, swiglu, max_ctas) + whole,
                  status_word(a.device).data_ptr(), _stream(),
                  tag=f"[{M}x{N}x{K}{'+swiglu' if swiglu else ''}]" if _native._timing is not None else "")
     return out
+
+
+def head_logits(a: torch.Tensor, w: torch.Tensor, vocab: int, scale: float = 1.0) -> torch.Tensor:
+    """fp32 logits ``gemm(a, w)[:, :vocab].float() * scale``; for few rows on CUDA the product writes them itself (the same
+    numbers, rounded to bf16 first)."""
+    M, K = a.shape
+    if (a.is_cuda and a.dtype == w.dtype == torch.bfloat16 and a.stride(1) == w.stride(1) == 1 and a.stride(0) % 8 == 0
+            and w.stride(0) % 8 == 0 and _native.load().tw_gemm_logits_takes(M, vocab, K)):
+        out = torch.empty(M, vocab, dtype=torch.float32, device=a.device)
+        _native.call("tw_gemm_logits", a.data_ptr(), a.stride(0), w.data_ptr(), w.stride(0), out.data_ptr(), vocab,
+                     float(scale), M, vocab, K, status_word(a.device).data_ptr(), _stream(),
+                     tag=f"[{M}x{vocab}x{K}]" if _native._timing is not None else "")
+        return out
+    out = gemm(a, w)[:, :vocab].float()
+    return out if scale == 1.0 else out * scale
 
 
 FP8 = torch.float8_e4m3fn

@@ -87,6 +87,8 @@ _SIGNATURES = {
                                 f32, vp, i32, f32, i32, i32, vp, i32, vp, ll, vp, vp],
     "tw_attn_decode_grouped": [vp, ll, vp, vp, i32, i32, vp, ll, vp, vp, vp, i32, vp, i32, i32, i32, i32, i32, f32, vp, i32,
                                f32, i32, i32, vp, i32, vp, ll, i32, vp, vp, vp, vp],
+    "tw_gemm_logits_takes": [i32, i32, i32],
+    "tw_gemm_logits": [vp, ll, vp, ll, vp, ll, f32, i32, i32, i32, vp, vp],
     "tw_gemm_bf16_act": [vp, ll, vp, ll, vp, ll, vp, i32, i32, i32, i32, i32, i32, i32, i32, vp, vp],
     "tw_gemm_bf16_clamped": [vp, ll, vp, ll, ll, vp, ll, vp, i32, i32, i32, f32, f32, i32, vp, vp, i32, i32, i32, i32, vp, vp],
     "tw_latent_prep": [vp, ll, i32, i32, vp, vp, ll, i32, i32, vp, i32, i32, vp, vp, vp, vp, i32, i32, f32, i32, vp],

@@ -452,14 +452,14 @@ def projection(x: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor], c
     """``out = x w^T + bias``, then ``act`` ("silu" or "relu2", the square of relu) on the columns ``[cols[0], cols[1])``
     (in the product's epilogue in bf16)."""
     if not x.is_cuda:
-        gemm(x, w, out=out, bias=bias)
+        gemm(x, w, out=out, bias=bias, cut_k=False)
         if cols is not None:
             part = out[:, cols[0]:cols[1]]
             part.copy_(torch.relu(part) ** 2 if act == "relu2" else torch.nn.functional.silu(part))
         return out
     if cols is None or x.dtype == torch.bfloat16:
-        return gemm(x, w, out=out, bias=bias, col_act=None if cols is None else (act, *cols))
-    gemm(x, w, out=out, bias=bias)
+        return gemm(x, w, out=out, bias=bias, col_act=None if cols is None else (act, *cols), cut_k=False)
+    gemm(x, w, out=out, bias=bias, cut_k=False)
     part = out[:, cols[0]:cols[1]]
     _native.call("tw_act_cols", part.data_ptr(), _row_stride(part), part.shape[0], part.shape[1], COL_ACTS[act], _dt(part),
                  _stream())
@@ -484,7 +484,7 @@ def gated_product(x: torch.Tensor, w: torch.Tensor, act: "str | tuple", out: tor
         ref.gated_product(x, w, act, out)
         return
     if x.dtype == torch.bfloat16:
-        gemm(x, w, out=out, swiglu=True, act=act)
+        gemm(x, w, out=out, swiglu=True, act=act, cut_k=False)
         return
     gemm(x, w, out=tmp)
     glu(tmp, act, out)
