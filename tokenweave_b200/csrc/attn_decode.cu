@@ -198,6 +198,8 @@ __global__ void __launch_bounds__(D)
 attn_decode_merge_kernel(const float* __restrict__ part_o, const float* __restrict__ part_ml,
                          const int* __restrict__ tok_row, int hq, int splits,
                          __nv_bfloat16* __restrict__ out, long long ldo) {
+  allow_dependents();                  // the product behind it may set up and fetch weights meanwhile
+  wait_predecessor();
   const int tok = blockIdx.x, h = blockIdx.y, d = threadIdx.x;
   const long long base = (static_cast<long long>(tok) * hq + h) * splits;
   float mm = -INFINITY;
@@ -222,7 +224,7 @@ extern "C" int tw_attn_decode_merge(const float* part_o, const float* part_ml, c
   if (n_tok <= 0 || splits <= 1) return 0;
   auto ob = reinterpret_cast<__nv_bfloat16*>(out);
   if (D == 128)
-    attn_decode_merge_kernel<128><<<dim3(n_tok, hq), 128, 0, stream>>>(part_o, part_ml, tok_row, hq, splits, ob, ldo);
+    launch_dependent(attn_decode_merge_kernel<128>, dim3(n_tok, hq), 128, 0, stream, part_o, part_ml, tok_row, hq, splits, ob, ldo);
   else if (D == 64)
     attn_decode_merge_kernel<64><<<dim3(n_tok, hq), 64, 0, stream>>>(part_o, part_ml, tok_row, hq, splits, ob, ldo);
   else {

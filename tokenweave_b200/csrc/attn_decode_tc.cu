@@ -149,6 +149,7 @@ attn_decode_tc_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_cons
   const int n_tiles = max(0, t_end - t_begin);
   auto tile_at = [&](int j) { return GROUPED && t_begin + j >= n_pre ? t_begin + j - n_pre + j_lo : t_begin + j; };
 
+  allow_dependents();                  // the product behind it may set up and fetch weights meanwhile
   if (threadIdx.x == 0) {
     for (int i = 0; i < DTC_RING; ++i) {
       mbar_init(&k_full[i], 1);

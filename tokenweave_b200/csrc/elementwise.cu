@@ -45,6 +45,7 @@ rope_kv_write_kernel(__nv_bfloat16* __restrict__ qkv, long long ld, const int* _
                      int hq, int hkv, int D, int write_k_back,
                      const __nv_bfloat16* __restrict__ q_norm_w, const __nv_bfloat16* __restrict__ k_norm_w,
                      float eps) {
+  wait_predecessor();
   const int t = blockIdx.x;
   const int pos = positions[t];
   const int slot = (slots != nullptr) ? slots[t] : -1;
@@ -209,10 +210,9 @@ extern "C" int tw_rope_kv_write(void* qkv, long long ld, const int* positions, c
     set_last_error("rope_kv_write: head_dim must be a multiple of 16 and the row stride of 8");
     return 1;
   }
-  rope_kv_write_kernel<false><<<T, 256, 0, stream>>>(reinterpret_cast<__nv_bfloat16*>(qkv), ld, positions, slots,
-                                                      cos_sin, reinterpret_cast<__nv_bfloat16*>(k_cache),
-                                                      reinterpret_cast<__nv_bfloat16*>(v_cache), hq, hkv, D,
-                                                      write_k_back, nullptr, nullptr, 0.f);
+  launch_dependent(rope_kv_write_kernel<false>, T, 256, 0, stream, reinterpret_cast<__nv_bfloat16*>(qkv), ld, positions, slots,
+                   cos_sin, reinterpret_cast<__nv_bfloat16*>(k_cache), reinterpret_cast<__nv_bfloat16*>(v_cache), hq, hkv, D,
+                   write_k_back, nullptr, nullptr, 0.f);
   return check_launch("rope_kv_write");
 }
 
@@ -227,7 +227,7 @@ extern "C" int tw_rope_kv_write_qknorm(void* qkv, long long ld, const int* posit
     set_last_error("rope_kv_write_qknorm: head_dim must be 16 * a power of two (<= 512), row stride a multiple of 8");
     return 1;
   }
-  rope_kv_write_kernel<true><<<T, 256, 0, stream>>>(
+  launch_dependent(rope_kv_write_kernel<true>, T, 256, 0, stream,
       reinterpret_cast<__nv_bfloat16*>(qkv), ld, positions, slots, cos_sin, reinterpret_cast<__nv_bfloat16*>(k_cache),
       reinterpret_cast<__nv_bfloat16*>(v_cache), hq, hkv, D, write_k_back,
       reinterpret_cast<const __nv_bfloat16*>(q_norm_w), reinterpret_cast<const __nv_bfloat16*>(k_norm_w), eps);

@@ -25,6 +25,8 @@ rmsnorm_kernel(__nv_bfloat16* __restrict__ x, __nv_bfloat16* __restrict__ res,
                __nv_bfloat16* __restrict__ out, const __nv_bfloat16* __restrict__ w, int T, int H,
                long long ldx, long long ldr, long long ldo, float eps) {
   __shared__ float scratch[32];
+  allow_dependents();                  // the product behind it may set up and fetch weights meanwhile
+  wait_predecessor();
   const int nvec = H >> 3;
   uint4 wv[VPT];
 #pragma unroll
@@ -122,7 +124,7 @@ static int launch_norm(void* x, void* res, void* out, const void* w, int T, int 
   auto wb = reinterpret_cast<const __nv_bfloat16*>(w);
 #define TW_NORM_CASE(V)                                                                         \
   case V:                                                                                       \
-    rmsnorm_kernel<V, MODE><<<grid, threads, 0, stream>>>(xb, rb, ob, wb, T, H, ldx, ldr, ldo, eps); \
+    launch_dependent(rmsnorm_kernel<V, MODE>, grid, threads, 0, stream, xb, rb, ob, wb, T, H, ldx, ldr, ldo, eps); \
     break;
   switch (vpt) {
     TW_NORM_CASE(1)

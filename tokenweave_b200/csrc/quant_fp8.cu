@@ -52,6 +52,8 @@ quant_fp8_kernel(const __nv_bfloat16* __restrict__ x, __nv_bfloat16* __restrict_
                  const __nv_bfloat16* __restrict__ w, uint8_t* __restrict__ out, float* __restrict__ scales,
                  int T, int H, long long ldx, long long ldr, long long ldo, float eps) {
   __shared__ float scratch[32];
+  allow_dependents();                  // the product behind it may set up and fetch weights meanwhile
+  wait_predecessor();
   const int nvec = H >> 3;
   uint4 wv[VPT];
   if (MODE != 0) {
@@ -176,7 +178,7 @@ static int launch_quant(const void* x, void* res, const void* w, void* out, floa
   auto ob = reinterpret_cast<uint8_t*>(out);
 #define TW_QUANT_CASE(V)                                                                              \
   case V:                                                                                             \
-    quant_fp8_kernel<V, MODE, DYNAMIC, INT8><<<grid, threads, 0, stream>>>(xb, rb, wb, ob, scales, T, H, ldx, \
+    launch_dependent(quant_fp8_kernel<V, MODE, DYNAMIC, INT8>, grid, threads, 0, stream, xb, rb, wb, ob, scales, T, H, ldx, \
                                                                            ldr, ldo, eps);                  \
     break;
   switch (vpt) {

@@ -29,4 +29,21 @@ bool make_tensor_map_u8(CUtensorMap* out, const void* base, int rank, const uint
 
 int device_sm_count();
 
+// A launch that may start while the kernel before it on the stream still runs (if that one calls allow_dependents); the kernel
+// calls wait_predecessor before it touches memory.
+template <typename... Params, typename... Args>
+inline cudaError_t launch_dependent(void (*kern)(Params...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, Args... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kern, static_cast<Params>(args)...);
+}
+
 }  // namespace tw
