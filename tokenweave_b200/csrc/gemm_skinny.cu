@@ -204,116 +204,116 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constan
   const uint32_t part0 = smem_u32(smem);
   constexpr int GROUPS = OUT / 8;
   for (int t0 = 0; t0 < p.tn; t0 += p.dump_rows) {
-  const int t1 = min(t0 + p.dump_rows, p.tn);
-  if (warp >= 2) {
-    // accumulators -> shared memory, [row of A][row of W]: lanes are rows of W, so a warp writes 128 bytes in a row
-    tc_fence_after_sync();
-    const int q = warp & 3;
-    float* dst = reinterpret_cast<float*>(smem) + q * 32 + lane;
-    const uint32_t src = tmem + (static_cast<uint32_t>(q * 32) << 16);
-    if (!abort_flag) {
+    const int t1 = min(t0 + p.dump_rows, p.tn);
+    if (warp >= 2) {
+      // accumulators -> shared memory, [row of A][row of W]: lanes are rows of W, so a warp writes 128 bytes in a row
+      tc_fence_after_sync();
+      const int q = warp & 3;
+      float* dst = reinterpret_cast<float*>(smem) + q * 32 + lane;
+      const uint32_t src = tmem + (static_cast<uint32_t>(q * 32) << 16);
+      if (!abort_flag) {
 #pragma unroll 1
-      for (int c = t0; c < t1; c += 16) {
-        uint32_t v[16];
-        tmem_ld_32x16(src + c, v);
-        tmem_wait_ld();
+        for (int c = t0; c < t1; c += 16) {
+          uint32_t v[16];
+          tmem_ld_32x16(src + c, v);
+          tmem_wait_ld();
 #pragma unroll
-        for (int j = 0; j < 16; ++j) dst[(c - t0 + j) * SK_ROWS] = __uint_as_float(v[j]);
+          for (int j = 0; j < 16; ++j) dst[(c - t0 + j) * SK_ROWS] = __uint_as_float(v[j]);
+        }
       }
+      tc_fence_before_sync();
     }
-    tc_fence_before_sync();
-  }
-  __syncthreads();
-  if (warp == 1 && t1 == p.tn) {
-    tc_fence_after_sync();
-    if (PAIR) tmem_dealloc_pair(tmem, p.tmem_cols);
-    else tmem_dealloc(tmem, p.tmem_cols);
-  }
-  if (p.split > 1) {
-    __syncwarp();
-    cluster_sync_all();
-  }
+    __syncthreads();
+    if (warp == 1 && t1 == p.tn) {
+      tc_fence_after_sync();
+      if (PAIR) tmem_dealloc_pair(tmem, p.tmem_cols);
+      else tmem_dealloc(tmem, p.tmem_cols);
+    }
+    if (p.split > 1) {
+      __syncwarp();
+      cluster_sync_all();
+    }
 
-  // ---- sums of the parts and epilogue: 8 neighbouring outputs of one row at a time ----
-  const int items = (min(t1, p.M) - t0) * GROUPS;
-  for (int i = part * SK_THREADS + threadIdx.x; i < items; i += p.split * SK_THREADS) {
-    const int row = i / GROUPS, g = i % GROUPS;
-    const int t = t0 + row, n = w0 + g * 8;
-    if (n >= p.N) continue;
-    float v[8], u[8];
+    // ---- sums of the parts and epilogue: 8 neighbouring outputs of one row at a time ----
+    const int items = (min(t1, p.M) - t0) * GROUPS;
+    for (int i = part * SK_THREADS + threadIdx.x; i < items; i += p.split * SK_THREADS) {
+      const int row = i / GROUPS, g = i % GROUPS;
+      const int t = t0 + row, n = w0 + g * 8;
+      if (n >= p.N) continue;
+      float v[8], u[8];
 #pragma unroll
-    for (int e = 0; e < 8; ++e) v[e] = u[e] = 0.f;
-    const uint32_t at = part0 + (row * SK_ROWS + g * 8) * 4;
-    for (int s = 0; s < p.split; ++s) {
+      for (int e = 0; e < 8; ++e) v[e] = u[e] = 0.f;
+      const uint32_t at = part0 + (row * SK_ROWS + g * 8) * 4;
+      for (int s = 0; s < p.split; ++s) {
 #pragma unroll
-      for (int h = 0; h < 2; ++h) {
-        float4 a;
-        if (p.split > 1) a = ld_cluster_f4(at + h * 16, s * CTAS + half);
-        else a = *reinterpret_cast<const float4*>(smem + (row * SK_ROWS + g * 8) * 4 + h * 16);
-        v[4 * h] += a.x; v[4 * h + 1] += a.y; v[4 * h + 2] += a.z; v[4 * h + 3] += a.w;
+        for (int h = 0; h < 2; ++h) {
+          float4 a;
+          if (p.split > 1) a = ld_cluster_f4(at + h * 16, s * CTAS + half);
+          else a = *reinterpret_cast<const float4*>(smem + (row * SK_ROWS + g * 8) * 4 + h * 16);
+          v[4 * h] += a.x; v[4 * h + 1] += a.y; v[4 * h + 2] += a.z; v[4 * h + 3] += a.w;
+          if (GLU) {
+            if (p.split > 1) a = ld_cluster_f4(at + OUT * 4 + h * 16, s * CTAS + half);
+            else a = *reinterpret_cast<const float4*>(smem + (row * SK_ROWS + OUT + g * 8) * 4 + h * 16);
+            u[4 * h] += a.x; u[4 * h + 1] += a.y; u[4 * h + 2] += a.z; u[4 * h + 3] += a.w;
+          }
+        }
+      }
+      const float rs = p.row_scale != nullptr ? p.row_scale[t] : 1.f;
+      float r[8];
+#pragma unroll
+      for (int e = 0; e < 8; ++e) {
+        const int c = min(n + e, p.N - 1);
         if (GLU) {
-          if (p.split > 1) a = ld_cluster_f4(at + OUT * 4 + h * 16, s * CTAS + half);
-          else a = *reinterpret_cast<const float4*>(smem + (row * SK_ROWS + OUT + g * 8) * 4 + h * 16);
-          u[4 * h] += a.x; u[4 * h + 1] += a.y; u[4 * h + 2] += a.z; u[4 * h + 3] += a.w;
+          float x = v[e], y = u[e];
+          if (FP8) {
+            x *= rs;
+            if (p.col_scale != nullptr) {
+              x *= p.col_scale[c];
+              y *= p.col_scale[p.up_row_offset + c];
+            }
+            r[e] = x / (1.f + __expf(-x)) * y * rs;
+          } else if (p.acts.glu == GLU_GELU_TANH) {
+            r[e] = epi_gelu_tanh(x) * y * rs;
+          } else if (p.acts.glu == GLU_CLAMPED) {
+            r[e] = epi_clamped(x * rs, y * rs, p.acts.limit, p.acts.alpha);
+          } else {
+            r[e] = x / (1.f + __expf(-x)) * y * rs;
+          }
+        } else {
+          float x = v[e];
+          if (FP8) {
+            x *= p.col_scale != nullptr ? rs * p.col_scale[c] : rs;
+            if (p.bias != nullptr) x += __bfloat162float(p.bias[c]);
+          } else {
+            if (p.bias != nullptr) x += __bfloat162float(p.bias[c]);
+            if (p.acts.col_act != 0 && c >= p.acts.col_begin && c < p.acts.col_end) {
+              const float z = fmaxf(x, 0.f);
+              x = p.acts.col_act == COL_RELU2 ? z * z : epi_silu(x);
+            }
+            x *= rs;
+          }
+          r[e] = x;
         }
       }
-    }
-    const float rs = p.row_scale != nullptr ? p.row_scale[t] : 1.f;
-    float r[8];
+      if (!GLU && p.logits != nullptr) {      // N is a multiple of 8 (checked by the launcher)
 #pragma unroll
-    for (int e = 0; e < 8; ++e) {
-      const int c = min(n + e, p.N - 1);
-      if (GLU) {
-        float x = v[e], y = u[e];
-        if (FP8) {
-          x *= rs;
-          if (p.col_scale != nullptr) {
-            x *= p.col_scale[c];
-            y *= p.col_scale[p.up_row_offset + c];
-          }
-          r[e] = x / (1.f + __expf(-x)) * y * rs;
-        } else if (p.acts.glu == GLU_GELU_TANH) {
-          r[e] = epi_gelu_tanh(x) * y * rs;
-        } else if (p.acts.glu == GLU_CLAMPED) {
-          r[e] = epi_clamped(x * rs, y * rs, p.acts.limit, p.acts.alpha);
-        } else {
-          r[e] = x / (1.f + __expf(-x)) * y * rs;
-        }
+        for (int e = 0; e < 8; ++e) r[e] = __bfloat162float(__float2bfloat16_rn(r[e])) * p.logit_scale;
+        float4* frow = reinterpret_cast<float4*>(p.logits + static_cast<long long>(t) * p.ldc + n);
+        frow[0] = make_float4(r[0], r[1], r[2], r[3]);
+        frow[1] = make_float4(r[4], r[5], r[6], r[7]);
+        continue;
+      }
+      __nv_bfloat16* crow = p.C + static_cast<long long>(t) * p.ldc + n;
+      if (n + 8 <= p.N) {
+        *reinterpret_cast<uint4*>(crow) = make_uint4(pack_bf16x2(r[0], r[1]), pack_bf16x2(r[2], r[3]),
+                                                     pack_bf16x2(r[4], r[5]), pack_bf16x2(r[6], r[7]));
       } else {
-        float x = v[e];
-        if (FP8) {
-          x *= p.col_scale != nullptr ? rs * p.col_scale[c] : rs;
-          if (p.bias != nullptr) x += __bfloat162float(p.bias[c]);
-        } else {
-          if (p.bias != nullptr) x += __bfloat162float(p.bias[c]);
-          if (p.acts.col_act != 0 && c >= p.acts.col_begin && c < p.acts.col_end) {
-            const float z = fmaxf(x, 0.f);
-            x = p.acts.col_act == COL_RELU2 ? z * z : epi_silu(x);
-          }
-          x *= rs;
-        }
-        r[e] = x;
+#pragma unroll
+        for (int e = 0; e < 8; ++e)
+          if (n + e < p.N) crow[e] = __float2bfloat16_rn(r[e]);
       }
     }
-    if (!GLU && p.logits != nullptr) {      // N is a multiple of 8 (checked by the launcher)
-#pragma unroll
-      for (int e = 0; e < 8; ++e) r[e] = __bfloat162float(__float2bfloat16_rn(r[e])) * p.logit_scale;
-      float4* frow = reinterpret_cast<float4*>(p.logits + static_cast<long long>(t) * p.ldc + n);
-      frow[0] = make_float4(r[0], r[1], r[2], r[3]);
-      frow[1] = make_float4(r[4], r[5], r[6], r[7]);
-      continue;
-    }
-    __nv_bfloat16* crow = p.C + static_cast<long long>(t) * p.ldc + n;
-    if (n + 8 <= p.N) {
-      *reinterpret_cast<uint4*>(crow) = make_uint4(pack_bf16x2(r[0], r[1]), pack_bf16x2(r[2], r[3]),
-                                                   pack_bf16x2(r[4], r[5]), pack_bf16x2(r[6], r[7]));
-    } else {
-#pragma unroll
-      for (int e = 0; e < 8; ++e)
-        if (n + e < p.N) crow[e] = __float2bfloat16_rn(r[e]);
-    }
-  }
-  if (t1 < p.tn) __syncthreads();
+    if (t1 < p.tn) __syncthreads();
   }
   if (CTAS * p.split > 1) {
     __syncwarp();
@@ -401,8 +401,8 @@ static bool skinny_pairs(int M, int N, bool glu) {
   return M > 112 && (M <= 160 ? 4 * tiles >= sms : tiles >= sms);
 }
 
-int gemm_skinny(bool fp8, bool cut, const void* A, long long lda, const void* W, long long ldw, long long rows_w, void* C, long long ldc,
-                const void* bias, const float* row_scale, const float* col_scale, int M, int N, int K, int glu,
+int gemm_skinny(bool fp8, bool cut, const void* A, long long lda, const void* W, long long ldw, long long rows_w, void* C,
+                long long ldc, const void* bias, const float* row_scale, const float* col_scale, int M, int N, int K, int glu,
                 int up_row_offset, const GemmActs& acts, uint32_t* status, cudaStream_t stream, float* logits,
                 float logit_scale) {
   const int esz = fp8 ? 1 : 2, bk = fp8 ? 128 : 64;
@@ -427,8 +427,8 @@ int gemm_skinny(bool fp8, bool cut, const void* A, long long lda, const void* W,
   const int slots = pairs ? 2 * sms : sms;
   const int enough = sms * (M < 64 ? 6 : 5) / 10;
   int split = 1;
-  while (cut && split * ctas * ctas < 8 && tile_ctas * split < enough && tile_ctas * split * 2 <= slots && p.num_kb / (split * 2) >= 4 &&
-         (!pair || dump <= two)) split *= 2;
+  while (cut && split * ctas * ctas < 8 && tile_ctas * split < enough && tile_ctas * split * 2 <= slots &&
+         p.num_kb / (split * 2) >= 4 && (!pair || dump <= two)) split *= 2;
   p.split = split;
   // One CTA per SM sets the pace itself: two k-blocks per stage halve its waits, as long as four stages are left
   // (fp8 5120x25600, 1 row: 37 -> 30 us; 100 rows, three stages: 46 -> 55 us).
